@@ -33,3 +33,18 @@ def test_log_and_reciprocal(lo, hi, eps):
         for c, v in ((1, X), (2, Y)):
             ref = -v / (2 * pi * r2)
             assert np.all(np.abs(np.abs(out[c]) - np.abs(ref)) <= 1e-12 * np.abs(ref) + 1e-300)
+
+
+@pytest.mark.parametrize("same", [True, False])
+@pytest.mark.parametrize("log2_eps", [508.5, 509.5, 510.75, 511.5])
+def test_large_eps(log2_eps, same):
+    """eps^2 up to and beyond the table's range: the potential is the charges' sum times log(eps^2) / (4 pi),
+    to a rounding a charge and 8 of the rest."""
+    import barytreek_b200 as btk
+    rng = np.random.default_rng(6)
+    n = 300
+    pts, q = (rng.random(n), rng.random(n)), rng.uniform(0.5, 1.0, n)
+    tc = btk.Treecode(pts, None if same else tuple(p[::-1].copy() for p in pts), degree=2, cluster_size=40, theta=0.7,
+                      eps=2.0 ** log2_eps, kind=btk.KIND_POT)
+    ref = float(q.sum()) * 2 * log2_eps * np.log(2.0) / (4 * np.pi)
+    assert np.all(np.abs(tc.solve(q).cpu().numpy()[0] - ref) <= (n + 8) * 2.0 ** -53 * ref)
