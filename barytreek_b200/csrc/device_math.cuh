@@ -72,37 +72,48 @@ __device__ __forceinline__ double rcp_fp64_pos_guarded(double x) {
 // ---------------------------------------------------------------------------
 // FP64 natural logarithm of a positive x in [2^-1022, 2^1021), for the 2-D kernels
 // (table-driven range reduction after Tang, ACM TOMS 16(4), 1990, with the
-// reciprocal from the FP32 unit): x = 2^e f, f in [1, 2); c = 1/f rounded to a
-// multiple of 2^-10, so u = x 2^-e c - 1 (one fma, exact to its rounding) is at
-// most 2^-10 and log x = e ln 2 - log c + log(1 + u), the last by its series
-// to u^5 (the rest is below 2^-62). -log c comes from a table of the 513
-// values of c in shared memory (log_table_fill). 10 FP64 operations; errors
-// stay near one rounding of the result (test_gpu_log2d.py). Non-finite x give
-// non-finite results. yf: the FP32 reciprocal of f, for a caller that needs
-// 1/x too (rcp_from_log).
+// reciprocal from the FP32 unit): x = 2^e f, f in [sqrt(1/2), sqrt(2)), so that
+// e ln 2 and log f never cancel (e = 0 for every x near 1); c = 1/f rounded to 9
+// mantissa bits, so u = x 2^-e c - 1 (one fma, exact to its rounding) is at most
+// h = 2^-10 and log x = e ln 2 - log c + log(1 + u). c is 1 and the table's value 0
+// where f is within 2^-11 of 1, so log x keeps its relative accuracy there. The
+// last by its series to u^6, the sixth term folded into the others by
+// u^4 = h^2 u^2 - h^4 / 8 (its Chebyshev polynomial left out): at most u^2 h^4 / 48
+// is lost. -log c comes from a table over the values of c in shared memory
+// (log_table_fill). 10 FP64 operations; the error is at most 2.6 roundings of the
+// result (0.7 rms; test_gpu_log2d.py). With f in [1, 2) instead x just below 1
+// lost up to 460. Non-finite x give non-finite results. yf: the FP32 reciprocal of
+// f, for a caller that needs 1/x too (rcp_from_log).
 // ---------------------------------------------------------------------------
-constexpr int kLogTable = 513;
+constexpr int kLogTable = 515;
+// c of table entry k, as the high word of a double, and entry 0 as FP32 bits.
+constexpr int kLogHi = 0x3fe69800;
+constexpr unsigned kLogFirst = 0x3f34c000u;
 
 __device__ __forceinline__ void log_table_fill(double* table) {
-  for (int k = threadIdx.x; k < kLogTable; k += blockDim.x) table[k] = -log(0.5 + k * 0.0009765625);
+  for (int k = threadIdx.x; k < kLogTable; k += blockDim.x) table[k] = -log(__hiloint2double(kLogHi + (k << 11), 0));
 }
 
+// The biased exponent e + 1023 of x = 2^e f, in place (sqrt(2) is 0x3ff6a09e...).
+__device__ __forceinline__ int log_exponent(double x) { return (__double2hiint(x) + (0x00100000 - 0x0006a09e)) & 0x7ff00000; }
+
 __device__ __forceinline__ double log_fp64_pos(double x, const double* table, float& yf) {
-  const int hi = __double2hiint(x), eb = hi & 0x7ff00000;
-  const unsigned fb = (__funnelshift_l(__double2loint(x), hi, 3) & 0x007fffffu) | 0x3f800000u;
+  const int eb = log_exponent(x);
+  const unsigned fb = __funnelshift_l(__double2loint(x), __double2hiint(x) - eb, 3) + 0x3f800000u;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__uint_as_float(fb)));
-  const unsigned k = (__float_as_uint(yf) - (0x3f000000u - 0x2000u)) >> 14;  // c = 1/2 + k / 1024
-  const double c = __hiloint2double((int)(k << 11) + 0x7fd00000 - eb, 0);   // c 2^-e
+  const unsigned k = (__float_as_uint(yf) - (kLogFirst - 0x2000u)) >> 14;
+  const double c = __hiloint2double((int)(k << 11) + (kLogHi + 0x3ff00000) - eb, 0);  // c 2^-e
   const double u = fma(x, c, -1.0), q = u * u;
-  const double a = fma(q, fma(u, 0.2, -0.25), fma(u, 1.0 / 3.0, -0.5));
-  const double e = __hiloint2double(0x43300000, eb >> 20) - (4503599627370496.0 + 1023.0);  // 2^52 + biased exponent
-  return fma(e, 0.693147180559945309417, table[k]) + fma(q, a, u);
+  constexpr double h2 = 0x1p-20;
+  const double a = fma(q, fma(u, 0.2, -0.25 - h2 / 6.0), fma(u, 1.0 / 3.0, -0.5 + h2 * h2 / 48.0));
+  const double e = __hiloint2double(0x43300000, eb) - (4503599627370496.0 + 1023.0 * 1048576.0);  // 2^20 e
+  return fma(e, 0.693147180559945309417 / 1048576.0, table[k]) + fma(q, a, u);
 }
 
 // 1 / x from log_fp64_pos's reciprocal: y 2^-e and one Newton step (rcp_fp64_pos).
 __device__ __forceinline__ double rcp_from_log(double x, float yf) {
   const double f = (double)yf;
-  const double y = __hiloint2double(__double2hiint(f) + 0x3ff00000 - (__double2hiint(x) & 0x7ff00000), __double2loint(f));
+  const double y = __hiloint2double(__double2hiint(f) + 0x3ff00000 - log_exponent(x), __double2loint(f));
   return fma(y, fma(-x, y, 1.0), y);
 }
 

@@ -48,3 +48,28 @@ def test_large_eps(log2_eps, same):
                       eps=2.0 ** log2_eps, kind=btk.KIND_POT)
     ref = float(q.sum()) * 2 * log2_eps * np.log(2.0) / (4 * np.pi)
     assert np.all(np.abs(tc.solve(q).cpu().numpy()[0] - ref) <= (n + 8) * 2.0 ** -53 * ref)
+
+
+@pytest.mark.parametrize("direct", [False, True])
+def test_relative_error_near_one(direct):
+    """r^2 around 1, exact in FP64 (x of 26 bits, y = 0): the logarithm keeps its relative accuracy through its
+    zero. 7 roundings: 3 of the logarithm, its table's value against the sum 2, the constant factor 2."""
+    import torch
+
+    import barytreek_b200 as btk
+    from barytreek_b200 import _lib
+    rng = np.random.default_rng(7)
+    j = np.concatenate([np.arange(-1500, 0), np.arange(1, 1500), rng.integers(-2 ** 22, 2 ** 22, 5000)])
+    x = 1.0 + (j[j != 0] * 2.0 ** -25)
+    t, s, q = (x, np.zeros_like(x)), (np.array([0.0, 3.0]), np.zeros(2)), np.array([1.0, 0.0])
+    if direct:
+        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        T, S, Q, out = [dev(a) for a in t], [dev(a) for a in s], dev(q), torch.empty(len(x), dtype=torch.float64, device="cuda")
+        p = _lib.ptr
+        _lib.check(_lib.load().btk_direct_sum(2, btk.KIND_POT, 2.0 ** -60, len(x), p(T[0]), p(T[1]), None, 2, p(S[0]),
+                                              p(S[1]), None, p(Q), p(out), None))
+        out = out.cpu().numpy()
+    else:
+        out = btk.Treecode(t, s, degree=2, cluster_size=9000, theta=0.7, eps=2.0 ** -60).solve(q).cpu().numpy()[0]
+    ref = 2 * np.log1p(np.asarray(x - 1.0, np.longdouble)) / (4 * np.longdouble("3.14159265358979323846264338327950288"))
+    assert np.max(np.abs((out - ref) / ref)) <= 7 * 2.0 ** -53
