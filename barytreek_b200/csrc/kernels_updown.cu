@@ -50,8 +50,10 @@ __device__ __forceinline__ void bary_basis(double (&L)[M], double x, const doubl
 }
 
 // The same basis for many points of one leaf: reciprocals from the FP32 unit
-// with a cubic step (rounded to FP64 but for the last bit) instead of 2 M
-// divisions. The basis does not change when x and the nodes are scaled, so
+// with a cubic step (1e-7 of a rounding from the rounded value) instead of 2 M
+// divisions, and quotients by the sum corrected by their remainders: the
+// division form's errors (0.85 to 1.36 roundings rms for 3 to 13 nodes; without
+// the correction 0.07 to 0.1 more). The basis does not change when x and the nodes are scaled, so
 // they come times `scale`, a power of two that makes the node range 1 to 2 and
 // keeps every difference inside the FP32 unit's range; a point nearer than that
 // to a node, or within the near-node test, and a panel without a usable scale
@@ -85,7 +87,10 @@ __device__ __forceinline__ void bary_basis_fast(double (&L)[M], double x, const 
   }
   const double r = rcp_signed(denom);
 #pragma unroll
-  for (int i = 0; i < M; ++i) L[i] *= r;
+  for (int i = 0; i < M; ++i) {
+    const double q = L[i] * r;
+    L[i] = fma(fma(-q, denom, L[i]), r, q);
+  }
 }
 
 // A panel's nodes and their scaled form in shared memory (all threads call it,
