@@ -341,9 +341,9 @@ btk_status btk_batch_create(btk_batch** out, const btk_batch_desc* desc, const d
   if (s != BTK_OK) return fail(s);
   const size_t n = (size_t)std::max<int64_t>(b->n_points, 1);
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMalloc(&b->d_xyz, sizeof(double) * n * F.dim);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_q, sizeof(double) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_out, sizeof(double) * n * b->ncomp);
+  cudaError_t e = alloc_or_release([&] { return cudaMalloc(&b->d_xyz, sizeof(double) * n * F.dim); });
+  if (e == cudaSuccess) e = alloc_or_release([&] { return cudaMalloc(&b->d_q, sizeof(double) * n); });
+  if (e == cudaSuccess) e = alloc_or_release([&] { return cudaMalloc(&b->d_out, sizeof(double) * n * b->ncomp); });
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_q, 0, sizeof(double) * n, st);
   const double* src[3] = {x, y, z};
   for (int d = 0; d < F.dim && e == cudaSuccess; ++d)

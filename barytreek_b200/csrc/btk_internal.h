@@ -42,6 +42,19 @@ btk_status set_error(btk_status s, const std::string& msg);
 btk_status cuda_error(cudaError_t e, const char* what);
 void count_launch(int n = 1);
 
+// Frees what the drop-in cache holds on the current device, but for the entry of
+// a call in progress; whether there was any.
+bool dropin_release();
+// An allocation; where the device is out of memory, once more after dropin_release.
+template <class F>
+cudaError_t alloc_or_release(F alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();  // not left for the next launch's check
+  if (dropin_release() && (e = alloc()) == cudaErrorMemoryAllocation) cudaGetLastError();
+  return e;
+}
+
 #define BTK_CUDA(call)                                            \
   do {                                                            \
     cudaError_t e_ = (call);                                      \

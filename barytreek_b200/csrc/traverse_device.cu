@@ -78,7 +78,8 @@ struct Arena2 {
   }
   template <class U>
   cudaError_t alloc(U** p, size_t n) {
-    cudaError_t e = cudaMallocAsync((void**)p, sizeof(U) * std::max<size_t>(n, 1), st);
+    cudaError_t e =
+        alloc_or_release([&] { return cudaMallocAsync((void**)p, sizeof(U) * std::max<size_t>(n, 1), st); });
     if (e == cudaSuccess) ptrs.push_back(*p);
     return e;
   }

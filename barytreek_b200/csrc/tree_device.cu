@@ -282,7 +282,8 @@ struct TreeScratch {
   }
   template <class T>
   cudaError_t alloc(T** p, size_t n) {
-    cudaError_t e = cudaMallocAsync((void**)p, sizeof(T) * std::max<size_t>(n, 1), st);
+    cudaError_t e =
+        alloc_or_release([&] { return cudaMallocAsync((void**)p, sizeof(T) * std::max<size_t>(n, 1), st); });
     if (e == cudaSuccess) ptrs.push_back(*p);
     return e;
   }

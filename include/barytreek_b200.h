@@ -204,8 +204,10 @@ btk_status btk_split_interactions(const btk_interact_pair* interaction_list, int
  * (computed on the device), so a tree rebuilt into the same buffers is noticed
  * and rebuilt. Calls are serialised by one process-wide lock. The cache holds
  * device memory (the least recently used of more than 6 entries go when all
- * hold more than 2 GiB) until btk_dropin_cache_clear (no reference
- * counterpart), which frees it. */
+ * hold more than 2 GiB, and of more than 48) until an allocation of this
+ * library does not fit, which frees the entries of that device not in use, or
+ * btk_dropin_cache_clear (no reference counterpart), which frees all. A host
+ * program whose own allocations need the memory calls it. */
 btk_status btk_dropin_cache_clear(void);
 
 /* src/upward_pass.hpp:7 */
