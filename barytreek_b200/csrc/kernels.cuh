@@ -160,7 +160,7 @@ cudaError_t launch_interact_mutual(int dim, int kind, const InteractParams& p, i
 cudaError_t launch_react_add(int ncomp, int n, const int* T_out, Ptr4 react, Ptr4 out, cudaStream_t s);
 int interact_blocks_per_sm(int dim, int kind, int precision, bool guard, int tile);
 // The direct sum's sources as double4 in their own order; *large (one device
-// word) says whether a coordinate is too large for the fast reciprocals.
+// word) says whether a coordinate or charge is too large for the fast reciprocals.
 cudaError_t launch_pack_sources(int n, const double* x, const double* y, const double* z, const double* q,
                                 double4* out, int* large, cudaStream_t s);
 // Slices of the sources the sum is split into (direct_slices); with more than

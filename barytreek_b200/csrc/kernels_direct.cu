@@ -1,9 +1,10 @@
 // FP64 direct sum over every (target, source) pair, target == source included
 // (src/direct_sum_impl.hpp:9-94). Used for accuracy measurement against the
 // treecode (the reference's examples do the same, e.g.
-// examples/example_poisson_3d.cpp:163-183). Its reciprocals and logarithm are
-// rounded to FP64 (a cubic step on the FP32 seed), independent of the
-// treecode's one-step reciprocal square root.
+// examples/example_poisson_3d.cpp:163-183). Its reciprocal square roots and
+// quotients are rounded to FP64 (a cubic step on the FP32 seed, a remainder),
+// where the treecode takes one Newton step; the 2-D logarithm is the treecode's
+// (log_fp64_pos, checked by itself in test_gpu_log2d.py).
 //
 // Bound: FP64 issue (18 FP64 operations a potential + gradient pair). A block
 // of 4 warps owns 64 targets, two per lane, and one slice of the sources, a
@@ -27,12 +28,13 @@ namespace {
 constexpr int kDirectWarps = 4;
 constexpr int kDirectTile = 64;
 constexpr int kDirectBlocksPerSm = 4;  // 123 registers without spills: 12.8 ms; 5 blocks 15.8, 6 blocks 14.1 (spills)
-// Coordinates up to here keep r^2 inside the seeds' range; a call with larger
-// ones (or infinities) takes IEEE square roots, divisions and CUDA's log.
-constexpr double kDirectCoordMax = 1.0e18;
+// Coordinates up to here keep r^2 inside the seeds' range, charges the
+// quotients' remainders finite; a call with larger ones (or infinities) takes
+// IEEE square roots, divisions and CUDA's log.
+constexpr double kDirectCoordMax = 1.0e18, kDirectChargeMax = 1.0e200;
 
-// 1 / sqrt(x) and 1 / x rounded to FP64: the seeds of rsqrt_fp64_scaled and
-// rcp_fp64_pos (relative error e below 2e-7) and a step with error e^3.
+// 1 / sqrt(x) rounded to FP64: the seed of rsqrt_fp64_scaled (relative error e
+// below 2e-7) and a step with error e^3.
 __device__ __forceinline__ double rsqrt_full(double x) {
   float yf;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(fp32_seed_arg(x)));
@@ -40,14 +42,13 @@ __device__ __forceinline__ double rsqrt_full(double x) {
   const double e = fma(-x, y * y, 1.0);
   return fma(y, e * fma(e, 0.375, 0.5), y);
 }
-__device__ __forceinline__ double rcp_step(double x, double y) {
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double rcp_full(double x) {
-  float yf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(fp32_seed_arg(x)));
-  return rcp_step(x, (double)yf);
+// w / x rounded to FP64: rcp_fp64_pos (error 4e-14) and the quotient's remainder.
+// |w| <= kDirectChargeMax, so nothing overflows. A rounded reciprocal times w has
+// one rounding more and one operation less: 10,000 targets x 1M sources, vector
+// kernel 10.3 -> 11.4 ms, 2-D potential + gradient 17.9 -> 18.9 ms.
+__device__ __forceinline__ double quotient(double w, double x) {
+  const double y = rcp_fp64_pos(x), q = w * y;
+  return fma(fma(-x, q, w), y, q);
 }
 
 // One pair; sums without the constant factor, as eval_fp64's. FAST: r^2 inside
@@ -62,12 +63,12 @@ __device__ __forceinline__ void direct_pair(double tx, double ty, double tz, con
     float yf = 0.f;
     acc[0] = fma(FAST ? log_fp64_pos(r2, log_table, yf) : log(r2), s.w, acc[0]);
     if (KIND == BTK_KIND_FIELD) {
-      const double g = FAST ? s.w * rcp_full(r2) : s.w / r2;
+      const double g = FAST ? quotient(s.w, r2) : s.w / r2;
       acc[1] = fma(dx, g, acc[1]);
       acc[2] = fma(dy, g, acc[2]);
     }
   } else if (KIND == BTK_KIND_VEL) {
-    const double g = FAST ? s.w * rcp_full(r2) : s.w / r2;
+    const double g = FAST ? quotient(s.w, r2) : s.w / r2;
     acc[0] = fma(dx, g, acc[0]);
     acc[1] = fma(dy, g, acc[1]);
     acc[2] = fma(dz, g, acc[2]);
@@ -178,14 +179,14 @@ __global__ void k_direct_reduce(int slices, int nc, int nt, const double* partia
 }
 
 // Packs (x, y, z, q) into double4 in the original source order; *large is set
-// when a coordinate exceeds kDirectCoordMax.
+// when a coordinate exceeds kDirectCoordMax or a charge kDirectChargeMax.
 __global__ void k_pack_sources(int n, const double* x, const double* y, const double* z, const double* q,
                                double4* out, int* large) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double4 s = make_double4(x[i], y[i], z ? z[i] : 0.0, q[i]);
   out[i] = s;
-  if (!(fmax(fabs(s.x), fmax(fabs(s.y), fabs(s.z))) <= kDirectCoordMax)) *large = 1;
+  if (!(fmax(fabs(s.x), fmax(fabs(s.y), fabs(s.z))) <= kDirectCoordMax) || !(fabs(s.w) <= kDirectChargeMax)) *large = 1;
 }
 
 }  // namespace

@@ -57,3 +57,33 @@ def test_non_finite(kind, oracle):
         assert np.array_equal(fine, np.isfinite(out[c]))
         assert np.array_equal(np.isnan(ref[c]), np.isnan(out[c]))
         assert np.linalg.norm((out[c] - ref[c])[fine]) <= 1e-13 * np.linalg.norm(ref[c][fine])
+
+
+@pytest.mark.parametrize("dim,kind", [(2, 2), (3, 1)])
+def test_quotients_are_rounded_once(dim, kind):
+    """One source, r^2 exact (whole numbers, eps 1): the vector sums are the rounded w / r^2 times x and the factor,
+    each product rounded, bit for bit."""
+    rng = np.random.default_rng(9)
+    t = rng.integers(-30000, 30000, (dim, 4001)).astype(np.float64)
+    r2 = (t * t).sum(0) + 1.0
+    factor = -1.0 / ((2.0 if dim == 2 else 4.0) * np.pi)
+    for w in (1.0, 3.0, float(rng.integers(1, 2 ** 40)), -1.0 / 3.0, 1e-200, 1e199, 1e250):
+        out = direct(dim, kind, 1.0, t, np.zeros((dim, 1)), np.array([w]))
+        for c in range(dim):
+            assert np.array_equal(out[len(out) - dim + c], t[c] * (w / r2) * factor), (w, c)
+
+
+@pytest.mark.parametrize("dim,kind", [(2, 0), (2, 2), (3, 0), (3, 1), (3, 2)])
+@pytest.mark.parametrize("bad", ["target inf", "target nan", "source inf", "source nan", "charge inf", "charge nan"])
+def test_non_finite_at_ordinary_eps(dim, kind, bad, oracle):
+    """Where eps lets the fast reciprocals be taken: the same results are infinite or not numbers."""
+    rng = np.random.default_rng(4)
+    t, s, q = rng.random((dim, 200)), rng.random((dim, 100)), rng.uniform(0.1, 1, 100)
+    what, v = bad.split()
+    {"target": t[0], "source": s[0], "charge": q}[what][70] = float(v)
+    with np.errstate(all="ignore"):
+        out, ref = direct(dim, kind, 1e-4, t, s, q), oracle.direct(dim, kind, 1e-4, t, s, q)
+        for c in range(len(ref)):
+            fine = np.isfinite(ref[c])
+            assert np.array_equal(np.isnan(ref[c]), np.isnan(out[c])) and np.array_equal(ref[c][~fine], out[c][~fine], equal_nan=True)
+            assert np.linalg.norm((out[c] - ref[c])[fine]) <= 1e-13 * np.linalg.norm(ref[c][fine])
