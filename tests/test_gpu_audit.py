@@ -150,3 +150,19 @@ def test_plain_solve_after_learned_uses_the_set_degrees(oracle):
     assert rel(out, oracle_solve(oracle, tc, 2, q)) <= 1e-12
     tc.close()
     fresh.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_fallback_2d(precision):
+    """A 2-D learned solve that cannot reach its tolerance gives the fixed-degree FP64 solve's result."""
+    import barytreek_b200 as btk
+    from barytreek_b200 import datagen, selector
+    pts, q = datagen.uniform_box(36, 30011, 2, -1.0, 1.0)
+    kw = dict(degree=6, cluster_size=150, theta=0.7, eps=1e-4, kind=2)
+    tc = btk.Treecode(pts, precision=precision, degree_mode=btk._lib.DEGREE_PER_PAIR, degree_min=4, leaf_far_pairs=True, **kw)
+    out, rep = tc.solve_learned(q, selector.Selector.load(kind=2), tol=1e-12, pair_tol=1.0)
+    assert rep["fell_back"] == 1, rep
+    plain = btk.Treecode(pts, **kw)
+    assert rel(out.cpu().numpy(), plain.solve(q).cpu().numpy()) <= 1e-12
+    plain.close()
+    tc.close()

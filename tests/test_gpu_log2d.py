@@ -73,3 +73,20 @@ def test_relative_error_near_one(direct):
         out = btk.Treecode(t, s, degree=2, cluster_size=9000, theta=0.7, eps=2.0 ** -60).solve(q).cpu().numpy()[0]
     ref = 2 * np.log1p(np.asarray(x - 1.0, np.longdouble)) / (4 * np.longdouble("3.14159265358979323846264338327950288"))
     assert np.max(np.abs((out - ref) / ref)) <= 7 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("lo,hi,eps", [(1e-3, 1e4, 1e-4), (1e17, 1e30, 1.0), (1e100, 1e150, 1.0)])
+def test_signed_field(lo, hi, eps):
+    """Both components with their signs, and radii beyond the FP32 range, where the reciprocal comes with the
+    logarithm's exponent: 1e-12 relative."""
+    import barytreek_b200 as btk
+    rng = np.random.default_rng(8)
+    r, a = np.exp(rng.uniform(np.log(lo), np.log(hi), 3001)), rng.uniform(0.0, 2.0 * np.pi, 3001)
+    x, y = r * np.cos(a), r * np.sin(a)
+    src = (np.array([0.0, lo, -lo]), np.array([0.0, lo, lo]))
+    tc = btk.Treecode((x, y), src, degree=2, cluster_size=5000, theta=0.7, eps=eps, kind=btk.KIND_FIELD)
+    out = tc.solve(np.array([1.0, 0.0, 0.0])).cpu().numpy()
+    X, Y, E = (np.asarray(v, np.longdouble) for v in (x, y, eps))
+    for c, v in ((1, X), (2, Y)):
+        ref = -v / (2 * np.longdouble("3.14159265358979323846264338327950288") * (X * X + Y * Y + E * E))
+        assert np.all(np.abs(out[c] - ref) <= 1e-12 * np.abs(ref))

@@ -109,3 +109,25 @@ def test_wait_limit_timeout_then_recovery():
     tc.set_wait_limit(-1)
     close(tc.solve(q).cpu().numpy(), ref)
     tc.last_timing()
+
+
+@pytest.mark.parametrize("dim,kind,n,leaf", [(3, 0, 30011, 290), (3, 2, 30011, 290), (3, 1, 30011, 290),
+                                             (2, 0, 40009, 129), (2, 2, 40009, 129)])
+@pytest.mark.parametrize("value", [0.0, np.inf, np.nan])
+def test_zero_and_non_finite_charges(dim, kind, n, leaf, value):
+    """Weight 0 fills idle lanes: charges that are 0 (every third), and one infinite or not a number among them, give
+    what the one-sided form gives."""
+    import barytreek_b200 as btk
+    from barytreek_b200 import datagen
+    pts, q = datagen.uniform_box(3, n, dim, 0.0, 1.0)
+    q = q.copy()
+    q[::3] = 0.0
+    q[n // 2] = value
+    tc = btk.Treecode(pts, degree=3, cluster_size=leaf, theta=0.6, eps=1e-4, kind=kind)
+    assert tc.stats()["evals_pp"] >= 50000000
+    a, b = tc.solve(q).cpu().numpy(), solve_one_sided(tc, q)
+    assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(a[np.isinf(a)], b[np.isinf(b)])
+    for c in range(len(b)):
+        fine = np.isfinite(b[c])
+        assert np.array_equal(fine, np.isfinite(a[c]))
+        assert np.linalg.norm((a[c] - b[c])[fine]) <= 1e-12 * np.linalg.norm(b[c][fine])
