@@ -27,13 +27,13 @@ static_assert(offsetof(btk_run_config, ker_eps) == 48, "RunConfig ker_eps offset
 
 namespace btk {
 
-// Degree limit of the device kernels (stack/shared arrays are sized by it).
 // Lower end of the FP64 reciprocal square root's domain (device_math.cuh): a
 // solve whose eps^2 is below it runs the guarded kernels.
 constexpr double kSeedMin = 2.350988701644575e-38;  // 2^-125
 // The factor its results carry: 4 sqrt(2).
 constexpr double kRsqrtScale = 5.65685424949238019521;
 
+// Degree limit of the device kernels (stack/shared arrays are sized by it).
 constexpr int kMaxDegree = 12;
 constexpr int kMaxNodes = kMaxDegree + 1;
 

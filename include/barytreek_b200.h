@@ -281,8 +281,9 @@ btk_status btk_direct_sum(int dim, int kind, double eps, int nt, const double* x
 
 /* btk_direct_sum without any device allocation. No counterpart in the
  * reference. Same arguments and bit-identical results; its scratch (the
- * packed sources) lives in a static device array, so ns is limited to
- * 262,144 (BTK_ERR_INVALID_ARGUMENT above that). For callers that cannot
+ * packed sources, 8 MiB, and the partial sums of their slices, 8 MiB) lives
+ * in a static device array, so ns is limited to 262,144
+ * (BTK_ERR_INVALID_ARGUMENT above that). For callers that cannot
  * allocate during the call: a host whose caching allocator has reserved the
  * device memory, or a time-stepping loop that cannot pay an allocation every
  * step. Returns once the work is enqueued on `stream` (on the current
@@ -408,7 +409,7 @@ btk_status btk_plan_destroy(btk_plan* plan);
 /* Work and memory figures of a plan. */
 typedef struct {
   int64_t evals_pp, evals_pc, evals_cp, evals_cc; /* kernel evaluations per class */
-  int64_t work_items;                             /* interaction work items */
+  int64_t work_items;                             /* interaction work items (both forms of the leaf pairs) */
   int64_t device_bytes;                           /* device memory the plan holds */
   int levels_target, levels_source;
   float build_ms_total; /* host wall time of btk_plan_create */
@@ -434,7 +435,12 @@ btk_status btk_cc_operator_groups(int dim, const void* panels_target, int n_targ
  * order, runs the upward pass, the interactions and the downward pass, and
  * writes out[ncomp][point_count_target] (OVERWRITTEN, original point order).
  * x/y/z_* and charges are device arrays in the caller's order; z may be NULL
- * in 2-D; target pointers may equal source pointers. */
+ * in 2-D; target pointers may equal source pointers, and should where they are
+ * the same points: an FP64 solve of a one-tree plan then evaluates leaf pairs
+ * once for both directions (copies of the arrays give the same result in 1.1 to
+ * 1.5 times the time).
+ * Sums of several work items are added in the order they finish, so two runs
+ * may differ in the last bits (about 1e-15 relative), small problems included. */
 btk_status btk_plan_execute(btk_plan* plan, const double* xt, const double* yt, const double* zt,
                             const double* xs, const double* ys, const double* zs, const double* charges,
                             double* out, btk_stream_t stream);

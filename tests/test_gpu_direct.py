@@ -1,5 +1,5 @@
-"""btk_direct_sum at the edges of its split (64 targets a tile, 8 warps a block,
-1 to 8 blocks a cluster, 32 sources at a time) and outside the fast
+"""btk_direct_sum at the edges of its split (64 targets a tile, 4 warps a block,
+slices of the sources added by a second kernel, 32 sources at a time) and outside the fast
 reciprocals' range, against the oracle's direct sum. Tolerance: 1e-13 relative
 L2 (FP64 sums of at most 20,000 terms in another order)."""
 import numpy as np
